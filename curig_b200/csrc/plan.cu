@@ -904,12 +904,15 @@ int plan_setpts(Plan *p, long long nrow, int nchan, const double *du, const doub
         const int s = plan_setpts_geometry(p, nrow, nchan, du, dv, dw, stride, h_freq);
         return s != OK ? s : plan_setpts_bin(p, p->st);
     };
-    const bool held = p->d_grid != nullptr;
+    const bool held = p && p->d_grid;
     int s = both();
     if (s == ERR_NOMEM && held) {                  // without what the last points left behind
         plan_release_points(p);
         s = both();
     }
+    // without points (unless the arguments were refused, which leaves the last
+    // ones) the plan holds no memory either
+    if (s != OK && p && !p->ready) plan_release_points(p);
     return s;
 }
 
