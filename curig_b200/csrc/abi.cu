@@ -534,6 +534,8 @@ extern "C" void curig_test_tile_wait(int64_t polls, int noissue) { set_tile_wait
 
 extern "C" void curig_test_gather_scratch(int on) { set_gather_scratch(on); }
 
+extern "C" void curig_test_sparse_interp(int n) { set_sparse_interp(n); }
+
 extern "C" int curig_destroy(curig_plan h) {
     if (!h) return OK;
     plan_destroy(h->p);

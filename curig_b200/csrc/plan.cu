@@ -340,6 +340,14 @@ void set_tile_wait(long long polls, int noissue) {
     g_tma_noissue.store(noissue ? 1 : 0);
 }
 
+// The interpolator's sparse threshold (DEFAULT_SPARSE_I) is not an option of the
+// calls; a test sets it (negative: the default).
+namespace {
+std::atomic<int> g_sparse_interp{-1};
+}
+
+void set_sparse_interp(int n) { g_sparse_interp.store(n); }
+
 // ms2dirty's weighted gather takes a scratch vis * wgt from the pool, or, when
 // that allocation fails (or a test turns the scratch off), gathers vis and wgt
 // in one pass.
@@ -756,7 +764,8 @@ retry_tiles:
     g.tx = tg.tx; g.ty = tg.ty; g.tz = tg.tz; g.zpad = tg.zpad; g.sub = tg.sub;
     const int sp = p->opt.sparse;
     g.sparse_n = sp < 0 ? 0 : sp > 0 ? sp : esize == 4 ? DEFAULT_SPARSE_N : DEFAULT_SPARSE_N64;
-    p->sparse_i = sp < 0 ? 0 : sp > 0 ? sp : DEFAULT_SPARSE_I;
+    const int si = g_sparse_interp.load();
+    p->sparse_i = sp < 0 ? 0 : si >= 0 ? si : DEFAULT_SPARSE_I;   // (sp's positive values are the spreader's)
     g.tpitch = (tg.tx + 2) & ~1;
     g.use_tma = 0;                          // set once the grid's TMA descriptor exists
     g.tma_polls = g_tma_polls.load();

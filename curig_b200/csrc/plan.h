@@ -31,7 +31,7 @@ struct Options {
     int grid_x = 0, grid_y = 0;   // oversampled grid along the nxdirty / nydirty axes (0: sigma rule)
     int bin_z = 0;                // w-planes per tile slab (0: automatic)
     int slabs = 1;                // row slabs of the sort (one-shot copy / compute pipeline), 1..MAX_SLABS
-    int sparse = 0;               // tile kernels: chunks below this skip the tile (0: automatic, < 0: never)
+    int sparse = 0;               // spreader: chunks below this skip the tile (0: automatic, < 0: never, interpolator too)
     int n3 = 0;                   // generic 3-D NUFFT: modes along the third axis (0: the gridder)
 };
 
@@ -272,6 +272,9 @@ void set_tile_wait(long long polls, int noissue);
 // on = 0: ms2dirty gathers vis and wgt in one pass (no vis * wgt scratch), as
 // when the scratch cannot be allocated; tests compare the two paths
 void set_gather_scratch(int on);
+// interpolator's sparse threshold of plans whose points are set afterwards
+// (negative: DEFAULT_SPARSE_I), for tests
+void set_sparse_interp(int n);
 // destroy the cached cuFFT handles no plan holds (returns how many); number cached
 int fft_cache_trim();
 int fft_cache_size();

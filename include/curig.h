@@ -87,10 +87,11 @@ typedef struct curig_opts {
                              dirty2ms downloads slab k while slab k+1 is interpolated);
                              0 = automatic (3 from 1 GiB of visibilities and weights,
                              2 from 384 MiB, else 1).  Plans ignore it. */
-    int sparse;           /* tile kernels: a chunk of fewer visibilities than this adds its
-                             taps straight to the grid (or reads them from it) instead of
-                             through a shared-memory tile (0: automatic, spreader 96 in FP32,
-                             32 in FP64, interpolator 16; negative: always the tile) */
+    int sparse;           /* tile spreaders: a chunk of fewer visibilities than this adds its
+                             taps straight to the grid instead of through a shared-memory tile
+                             (0: automatic, 96 in FP32, 32 in FP64; negative: always the tile,
+                             also in the interpolator, which otherwise reads the grid directly
+                             for chunks below 16) */
 } curig_opts;
 
 void curig_default_opts(curig_opts *opts);
@@ -244,6 +245,12 @@ void curig_test_tile_wait(int64_t polls, int noissue);
  * in input order first.  The two differ only in the rounding order of the
  * products.  No counterpart in the reference. */
 void curig_test_gather_scratch(int on);
+
+/* Test hook for the interpolator's direct reads: plans whose points are set
+ * after this call interpolate chunks of fewer than n visibilities without a
+ * tile, unless curig_opts.sparse is negative; n < 0 restores the default (16),
+ * which curig_opts.sparse > 0 does not change.  No counterpart in the reference. */
+void curig_test_sparse_interp(int n);
 
 /* Generic NUFFT, types 1 (points -> modes) and 2 (modes -> points) in one or two
  * dimensions, on the w-free gridder (same kernel-width, grid-size and correction
