@@ -642,7 +642,7 @@ k_spread(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__ b
     if (g.wkind == 1)
         for (int i = threadIdx.x; i < kw * (g.wdeg + 1); i += NTHREADS) coef[i] = (T)wcoef[i];
     const int total = g.sub_hi ? g.sub_hi : sub_end[g.nbins - 1];   // sub-problem window [sub_lo, total)
-    const int kk = kw * kw, k3 = kk * kw;
+    const int kk = kw * kw, k3 = g.no_w ? kk : kk * kw;      // (w-free: one plane, no z taps)
     const int txy = g.tx * g.ty;
     for (int s = g.sub_lo + blockIdx.x; s < total; s += gridDim.x) {
         long long b = g.cbin ? g.cbin[s] : find_bin(sub_end, g.nbins, s);
@@ -665,7 +665,7 @@ k_spread(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__ b
                 int rm = t - dz * kk;
                 int dy = rm / kw;
                 int dx = rm - dy * kw;
-                T wt = ks[dx] * ks[KSTR + dy] * ks[2 * KSTR + dz];
+                T wt = ks[dx] * ks[KSTR + dy] * (g.no_w ? (T)1 : ks[2 * KSTR + dz]);
                 C<T> *p = tile + base + dz * txy + dy * g.tx + dx;
                 atomicAdd(&p->x, c.x * wt);
                 atomicAdd(&p->y, c.y * wt);
@@ -712,7 +712,7 @@ k_interp(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__ b
     if (g.wkind == 1)
         for (int i = threadIdx.x; i < kw * (g.wdeg + 1); i += NTHREADS) coef[i] = (T)wcoef[i];
     const int total = g.sub_hi ? g.sub_hi : sub_end[g.nbins - 1];   // sub-problem window [sub_lo, total)
-    const int kk = kw * kw, k3 = kk * kw;
+    const int kk = kw * kw, k3 = g.no_w ? kk : kk * kw;      // (w-free: one plane, no z taps)
     const int txy = g.tx * g.ty;
     for (int s = g.sub_lo + blockIdx.x; s < total; s += gridDim.x) {
         long long b = g.cbin ? g.cbin[s] : find_bin(sub_end, g.nbins, s);
@@ -746,7 +746,7 @@ k_interp(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__ b
                 int rm = t - dz * kk;
                 int dy = rm / kw;
                 int dx = rm - dy * kw;
-                T wt = ks[dx] * ks[KSTR + dy] * ks[2 * KSTR + dz];
+                T wt = ks[dx] * ks[KSTR + dy] * (g.no_w ? (T)1 : ks[2 * KSTR + dz]);
                 C<T> v = tile[base + dz * txy + dy * g.tx + dx];
                 ar = fma(v.x, wt, ar);
                 ai = fma(v.y, wt, ai);
@@ -1707,7 +1707,7 @@ __global__ void __launch_bounds__(interp_threads<T>(), sizeof(T) == 4 ? 3 : 2)
 k_interp_t(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__ bin_count,
            const int *__restrict__ sub_end, const R<T> *__restrict__ rec, const C<T> *__restrict__ grid,
            const WinTab<T> tab, const VisIO io, const __grid_constant__ CUtensorMap tmap, int *err) {
-    // FP32 windows of these widths are always tabulated (set points); said here,
+    // FP32 windows are always tabulated in this kernel (CURIG_KW_SWITCH); said here,
     // it takes win_tap's test and the direct form out of the tap loop: 6.4e7
     // visibilities, width 6, 6.32 -> 6.15 ms; 2e6 343 -> 328 us.  (The spreader
     // measured 9.52 -> 9.96 ms so, and keeps the test.)
@@ -2471,8 +2471,10 @@ static int launch_interp_kw(const DevGeom &g, size_t smem, const int *bs, const 
     return OK;
 }
 
+// The thread-per-visibility kernels by width; the general ones (0) for wider
+// windows and for learned tables beyond degree TAB_DEG - 1, which WinTab does not hold.
 #define CURIG_KW_SWITCH(F, ...)                                  \
-    switch (g.kw) {                                              \
+    switch (g.wdeg < TAB_DEG ? g.kw : 0) {                       \
     case 2: return F<T, 2>(__VA_ARGS__);                         \
     case 3: return F<T, 3>(__VA_ARGS__);                         \
     case 4: return F<T, 4>(__VA_ARGS__);                         \

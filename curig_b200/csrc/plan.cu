@@ -278,9 +278,8 @@ static std::vector<double> psi_terms(const KernelParams &kp, const Window &win, 
     return t;
 }
 
-// A learned window's table, leading zeros up to TAB_DEG columns; none beyond that degree.
+// A learned window's table (degree <= TAB_DEG - 1), leading zeros up to TAB_DEG columns.
 static std::shared_ptr<const WindowTable> learned_table(const Window &w) {
-    if (w.degree > TAB_DEG - 1) return nullptr;
     auto t = std::make_shared<WindowTable>();
     t->c.assign((size_t)w.kw * TAB_DEG, 0.0);
     for (int d = 0; d < w.kw; ++d)
@@ -463,6 +462,12 @@ static int tile_mode(const Plan *p) {
     }
 }
 
+// Does the window fit the thread-per-visibility kernels' tables?  Wider ones and
+// learned windows of a higher degree take the general kernels (k_spread, k_interp).
+static bool tabulated(const Plan *p) {
+    return p->gp.kp.kw <= TAB_KW && (p->win.kind == 0 || p->win.degree <= TAB_DEG - 1);
+}
+
 static int choose_tiles(Plan *p, int esize, bool force_slabs) {
     const GridParams &gp = p->gp;
     const int kw = gp.kp.kw;
@@ -470,7 +475,7 @@ static int choose_tiles(Plan *p, int esize, bool force_slabs) {
     // FP32 spreader: int32 fixed point, two words (exact) or one word per component;
     // FP64: three-word int32 fixed point (exact)
     const int mode = tile_mode(p);
-    t.fix = kw > TAB_KW ? 0 : esize == 4 ? (mode == 0 ? 1 : mode == 2 ? 2 : 0) : (mode != 1 ? 3 : 0);
+    t.fix = !tabulated(p) ? 0 : esize == 4 ? (mode == 0 ? 1 : mode == 2 ? 2 : 0) : (mode != 1 ? 3 : 0);
     // FP32 tiles: two CTAs per SM (<= 112 KB each); FP64 fixed-point tiles: one
     // CTA per SM (its registers), so a larger tile with less halo
     size_t budget = p->opt.smem_budget ? p->opt.smem_budget
@@ -621,7 +626,7 @@ int plan_setpts_geometry(Plan *p, long long nrow, int nchan, const double *du, c
     req.no_w = p->opt.w_term == 1 || p->opt.n3 > 0;
     int s = grid_params(p->nx, p->ny, p->psx, p->psy, lo, hi, p->eps, p->sigma, p->sign, p->gp, kw_override, req);
     if (s != OK) return s;
-    if (req.no_w && p->gp.kp.kw > TAB_KW) return ERR_UNSUPPORTED;   // thread-per-visibility kernels only
+    if (req.no_w && p->gp.kp.kw > TAB_KW) return ERR_UNSUPPORTED;   // no w-free mode at these widths
     if (p->opt.n3 > 0) {        // generic 3-D NUFFT: a periodic third axis of the NUFFT's own size
         GridParams &g3 = p->gp;
         g3.no_w = 0;
@@ -772,7 +777,8 @@ retry_tiles:
     g.tma_test_noissue = g_tma_noissue.load();
     // row slabs (tile kernels only): bins of slab k are k * nbins_slab + bin
     int nslab = std::max(1, std::min(p->opt.slabs, MAX_SLABS));
-    if (g.kw > TAB_KW || nrow < nslab || (long long)nslab * tg.nbins() > INT_MAX / 2) nslab = 1;
+    const bool tab = tabulated(p);
+    if (!tab || nrow < nslab || (long long)nslab * tg.nbins() > INT_MAX / 2) nslab = 1;
     p->nslab = nslab;
     g.nslab = nslab;
     g.nbins_slab = tg.nbins();
@@ -788,10 +794,10 @@ retry_tiles:
     // FP32 the ES window as degree-(TAB_DEG-1) Horner polynomials, in FP64 its
     // inner intervals at degree TAB64_DEG-1
     p->wtab.reset();
-    if (g.kw <= TAB_KW) {
+    if (tab) {
         if (p->win.kind == 1) p->wtab = learned_table(p->win);
         else p->wtab = es_table(gp.kp, p->opt.precision != 0);
-        if (p->wtab && (p->win.kind == 1 || p->opt.precision)) g.wkind = 1;
+        if (p->win.kind == 1 || p->opt.precision) g.wkind = 1;
     }
     // bounds on the window (sampled table maxima, 1% margin): per tap index d
     // over all offsets (wenv), of one tap's product (wmax3) and of the z factor;
@@ -821,7 +827,7 @@ retry_tiles:
     while ((1LL << binbits) < nb) ++binbits;
     // start-cell residue in the key: mod 16 for the FP32 tile kernels (their
     // class schedule needs it), mod 32 for the FP64 ones (bin-only keys beyond 31 bits)
-    const bool f32tile = esize == 4 && g.kw <= TAB_KW;
+    const bool f32tile = esize == 4 && tab;
     int cbits = f32tile ? 4 : (binbits + 5 <= 31 ? 5 : 0);
     if (binbits > 31 || binbits + cbits > 31) return ERR_UNSUPPORTED;
     g.cbits = cbits;

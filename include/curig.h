@@ -147,7 +147,8 @@ int curig_plan_error(curig_plan plan, double *est);
 /* ---------------------------------------------------------------- learned window
  * Register a piecewise-polynomial window for support width kw: coef is
  * [kw][degree+1], interval d covers t in [d - kw/2, d + 1 - kw/2], variable
- * s = 2 (t - d + kw/2) - 1 in [-1, 1], highest power first.  eps_reached is
+ * s = 2 (t - d + kw/2) - 1 in [-1, 1], highest power first; kw 2 .. 28, degree
+ * 1 .. 15 (beyond width 12 or degree 11 on slower kernels).  eps_reached is
  * the relative error the window reaches against the exact DFT; a plan with
  * opts.window = 1 picks the narrowest registered window with
  * eps_reached <= epsilon.  No counterpart in the reference (its kernel is the
