@@ -141,6 +141,8 @@ lib.curig_test_gather_scratch.argtypes = [c_int]
 lib.curig_test_gather_scratch.restype = None
 lib.curig_test_sparse_interp.argtypes = [c_int]
 lib.curig_test_sparse_interp.restype = None
+lib.curig_test_ranked_bytes.argtypes = [c_int64]
+lib.curig_test_ranked_bytes.restype = None
 
 ERRORS = {
     1: "generic error", 2: "bad upsampling factor", 3: "invalid argument", 4: "CUDA error",

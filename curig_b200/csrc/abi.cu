@@ -536,6 +536,8 @@ extern "C" void curig_test_gather_scratch(int on) { set_gather_scratch(on); }
 
 extern "C" void curig_test_sparse_interp(int n) { set_sparse_interp(n); }
 
+extern "C" void curig_test_ranked_bytes(int64_t n) { set_ranked_bytes(n); }
+
 extern "C" int curig_destroy(curig_plan h) {
     if (!h) return OK;
     plan_destroy(h->p);

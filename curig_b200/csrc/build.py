@@ -6,8 +6,9 @@ Objects go to curig_b200/csrc/_build/, the shared library to
 curig_b200/libcurafft.so (next to the Python package, as the reference's
 package_data, setup.py:24).  --check builds the bounds-checked variant
 curig_b200/libcurafft_check.so (objects in _build_check/, -DCURIG_BOUNDS_CHECK:
-the kernels check their buffer indices, skip an access that would leave its
-buffer and report it as an error status); select it with CURIG_LIB.
+the binning, tile, correction and row-pass kernels check their buffer indices,
+skip an access that would leave its buffer and report it as an error status);
+select it with CURIG_LIB.
 """
 from __future__ import annotations
 

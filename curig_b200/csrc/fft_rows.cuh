@@ -355,6 +355,19 @@ __device__ __forceinline__ double2 ld_once(const double2 *p, bool on) {
     return v;
 }
 
+// The buffers that a launch reads and writes, for the index checks of the
+// bounds-checked build (nothing of it is left in the regular one): n elements at
+// p, aligned to their size, inside the buffer.
+template <typename T> struct Limits {
+    const C<T> *in0, *in1, *out0, *out1;
+    int *flags;
+    __device__ __forceinline__ static bool inside(const C<T> *p, int n, const C<T> *a, const C<T> *b) {
+        return p >= a && p + n <= b && (size_t)p % (n * sizeof(C<T>)) == 0;
+    }
+    __device__ __forceinline__ bool reads(const C<T> *p, int n) const { return inside(p, n, in0, in1); }
+    __device__ __forceinline__ bool writes(const C<T> *p, int n) const { return inside(p, n, out0, out1); }
+};
+
 // Where a unit comes from and goes to: element i of its row (FP64) or of its
 // two rows (FP32; the second `row2` elements after the first, absent where two
 // is false).  In T the X passes' two rows are neighbours (y, y + 1).
@@ -367,7 +380,9 @@ template <typename T, bool X, int SP> struct RowMem {
     bool two, act, m2d, odd;       // odd: SP = 2, the odd outputs
     int lo, hi, m;                 // elements outside the image: [lo, hi); row length of T
     int w0, w1;                    // elements of the grid side inside the window
+    Limits<T> lim;
     __device__ __forceinline__ Cx<S> row(int i, bool on) const {
+        on = on && IN_BOUNDS(lim.reads(in + i, 1) && lim.reads(in + i + row2, 1), lim.flags);
         if constexpr (sizeof(T) == 8) {
             const C<T> u = ld_once(in + i, on);
             return Cx<S>{u.x, u.y};
@@ -378,6 +393,7 @@ template <typename T, bool X, int SP> struct RowMem {
     }
     __device__ __forceinline__ Cx<S> col(int i, bool on) const {
         const C<T> *a = in + (long long)(i < lo ? i : i - hi + lo) * m;
+        on = on && IN_BOUNDS(lim.reads(a, 16 / (int)sizeof(C<T>)), lim.flags);
         if constexpr (sizeof(T) == 8) {
             const C<T> u = ld_once(a, on);
             return Cx<S>{u.x, u.y};
@@ -387,6 +403,7 @@ template <typename T, bool X, int SP> struct RowMem {
         }
     }
     __device__ __forceinline__ void put_row(int i, Cx<S> v) const {
+        if (!IN_BOUNDS(lim.writes(out + i, 1) && lim.writes(out + i + row2, 1), lim.flags)) return;
         if constexpr (sizeof(T) == 8) out[i] = C<T>{v.x, v.y};
         else {
             float4 u;
@@ -398,6 +415,7 @@ template <typename T, bool X, int SP> struct RowMem {
     }
     __device__ __forceinline__ void put_col(int i, Cx<S> v) const {
         C<T> *o = out + (long long)(i < lo ? i : i - hi + lo) * m;
+        if (!IN_BOUNDS(lim.writes(o, 16 / (int)sizeof(C<T>)), lim.flags)) return;
         if constexpr (sizeof(T) == 8) *o = C<T>{v.x, v.y};
         else {
             float4 u;
@@ -520,6 +538,8 @@ k_fft_rows(int m2d, FftGeom g, const Cx<typename lane_t<T>::type> *__restrict__ 
     Cx<S> *sm = reinterpret_cast<Cx<S> *>(smem) + grp * L::pitch * L::F + f;
     const long long want = (((long long)(blockIdx.x / L::SP) * L::G + grp) * L::F + f) * PER;
     RowMem<T, L::x, L::SP> mem;
+    const long long ncell = (long long)g.nf3 * g.nf2 * g.nf1, nt = (long long)g.nf3 * g.ny * g.nf2;
+    mem.lim = Limits<T>{src, src + (L::x && m2d ? ncell : nt), dst, dst + (L::x && !m2d ? ncell : nt), g.dbg};
     mem.act = t < L::T && want < rows;                 // (idle threads read a unit again and write nothing)
     const long long row = want < rows ? want : 0;
     mem.m2d = m2d != 0;
@@ -563,6 +583,7 @@ template <typename T> struct ZMem {
     const double *psi3;
     double den;
     bool m2d, act;
+    Limits<T> lim;
     // mode index of grid index i, or -1
     __device__ __forceinline__ int mode(int i) const {
         return i < n3 - n3 / 2 ? i + n3 / 2 : i >= nf3 - n3 / 2 ? i - nf3 + n3 / 2 : -1;
@@ -574,14 +595,16 @@ template <typename T> struct ZMem {
         if (m2d) {
 #pragma unroll
             for (int q = 0; q < R; ++q) {
-                const C<T> u = ld_once(in + (j + q * STEP) * plane, true);
+                const C<T> *a = in + (j + q * STEP) * plane;
+                const C<T> u = ld_once(a, IN_BOUNDS(lim.reads(a, 1), lim.flags));
                 v[q] = Cx<double>{(double)u.x, (double)u.y};
             }
         } else {
 #pragma unroll
             for (int q = 0; q < R; ++q) {
                 const int iz = mode(j + q * STEP);
-                const C<T> u = ld_once(in + (iz < 0 ? 0 : iz), iz >= 0);
+                const C<T> *a = in + (iz < 0 ? 0 : iz);
+                const C<T> u = ld_once(a, iz >= 0 && IN_BOUNDS(lim.reads(a, 1), lim.flags));
                 const double w = iz < 0 ? 0.0 : 1.0 / corr(iz);
                 v[q] = Cx<double>{(double)u.y * w, (double)u.x * w};      // swapped: the forward direction
             }
@@ -592,13 +615,16 @@ template <typename T> struct ZMem {
 #pragma unroll
             for (int q = 0; q < R; ++q) {
                 const int iz = mode(j + q * STEP);
-                if (iz < 0) continue;
+                if (iz < 0 || !IN_BOUNDS(lim.writes(out + iz, 1), lim.flags)) continue;
                 const double d = corr(iz);
                 out[iz] = C<T>{(T)(v[q].x / d), (T)(v[q].y / d)};
             }
         } else {
 #pragma unroll
-            for (int q = 0; q < R; ++q) out[(j + q * STEP) * plane] = C<T>{(T)v[q].y, (T)v[q].x};
+            for (int q = 0; q < R; ++q) {
+                C<T> *o = out + (j + q * STEP) * plane;
+                if (IN_BOUNDS(lim.writes(o, 1), lim.flags)) *o = C<T>{(T)v[q].y, (T)v[q].x};
+            }
         }
     }
 };
@@ -626,6 +652,8 @@ k_fft_z(int m2d, DevCorr cc, const Cx<double> *__restrict__ tw, const C<T> *src,
     mem.plane = (long long)cc.ny * cc.nf2;
     mem.n3 = cc.n3;
     mem.nf3 = L::N;
+    const long long nt = mem.plane * L::N, nm = units * cc.n3;
+    mem.lim = Limits<T>{src, src + (m2d ? nt : nm), dst, dst + (m2d ? nm : nt), cc.dbg};
     mem.psi3 = cc.psi3;
     mem.den = cc.psi1[ks] * cc.psi2[kr];
     static_for<L::stages>([&](auto k) { fft_stage<L, decltype(k)::v>(t, tw, sm, mem); });

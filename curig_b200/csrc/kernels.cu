@@ -660,6 +660,7 @@ k_spread(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__ b
             __syncwarp();
             int cb = cell_bits(r.w);
             int base = ((cb >> 20) & 0xfff) * txy + ((cb >> 10) & 0x3ff) * g.tx + (cb & 0x3ff);
+            if (!IN_BOUNDS(base >= 0 && base + (k3 / kk - 1) * txy + (kw - 1) * (g.tx + 1) < ntile, g.dbg)) continue;
             for (int t = lane; t < k3; t += 32) {
                 int dz = t / kk;
                 int rm = t - dz * kk;
@@ -685,7 +686,10 @@ k_spread(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__ b
             const C<T> *trow = tile + row * g.tx;
             for (int x = lane; x < g.tx; x += 32) {
                 C<T> v = trow[x];
-                if (v.x != (T)0 || v.y != (T)0) atomic_add_c(grow + wrap3(ox + x, g.nf1), v);
+                const int gx = wrap3(ox + x, g.nf1);
+                if ((v.x != (T)0 || v.y != (T)0) &&
+                    IN_BOUNDS(gx >= 0 && gx < g.nf1 && gy >= 0 && gy < g.nf2 && gz >= 0 && gz < g.nf3, g.dbg))
+                    atomic_add_c(grow + gx, v);
             }
         }
         __syncthreads();
@@ -731,7 +735,11 @@ k_interp(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__ b
             int gz = g.zpad ? wrap3(oz + z, g.nf3) : z;
             const C<T> *grow = grid + ((long long)gz * g.nf2 + gy) * g.nf1;
             C<T> *trow = tile + row * g.tx;
-            for (int x = lane; x < g.tx; x += 32) trow[x] = grow[wrap3(ox + x, g.nf1)];
+            for (int x = lane; x < g.tx; x += 32) {
+                const int gx = wrap3(ox + x, g.nf1);
+                trow[x] = IN_BOUNDS(gx >= 0 && gx < g.nf1 && gy >= 0 && gy < g.nf2 && gz >= 0 && gz < g.nf3, g.dbg)
+                              ? grow[gx] : C<T>{0, 0};
+            }
         }
         __syncthreads();
         for (int i = first + warp; i < last; i += NWARPS) {
@@ -740,6 +748,7 @@ k_interp(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__ b
             __syncwarp();
             int cb = cell_bits(r.w);
             int base = ((cb >> 20) & 0xfff) * txy + ((cb >> 10) & 0x3ff) * g.tx + (cb & 0x3ff);
+            if (!IN_BOUNDS(base >= 0 && base + (k3 / kk - 1) * txy + (kw - 1) * (g.tx + 1) < ntile, g.dbg)) continue;
             T ar = 0, ai = 0;
             for (int t = lane; t < k3; t += 32) {
                 int dz = t / kk;
@@ -2255,11 +2264,13 @@ __global__ void __launch_bounds__(256) k_t_to_grid(int ny, int nf1, int nf2, con
 // Zero the window [x0, x1) x [y0, y1) of every grid plane (16-byte stores: x0
 // and the width are even).
 template <typename T>
-__global__ void k_zero_window(int nf1, int nf2, int x0, int y0, int w, int h, long long nrows, C<T> *__restrict__ grid) {
+__global__ void k_zero_window(int nf1, int nf2, int nf3, int x0, int y0, int w, int h, long long nrows,
+                              C<T> *__restrict__ grid, int *dbg) {
     const int n4 = (int)(w * sizeof(C<T>) / 16);
     for (long long r = blockIdx.x; r < nrows; r += gridDim.x) {
         const long long z = r / h, y = y0 + (r - z * h);
         float4 *row = reinterpret_cast<float4 *>(grid + (z * nf2 + y) * nf1 + x0);
+        if (!IN_BOUNDS(z < nf3 && y0 >= 0 && y < nf2 && x0 >= 0 && x0 + w <= nf1 && (size_t)row % 16 == 0, dbg)) continue;
         for (int k = threadIdx.x; k < n4; k += blockDim.x) row[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
@@ -2583,11 +2594,12 @@ void launch_zero_tpad(int nx, int ny, int nf2, int nf3, void *t, cudaStream_t st
 }
 
 template <typename T>
-void launch_zero_window(int nf1, int nf2, int nf3, int x0, int x1, int y0, int y1, void *grid, cudaStream_t st) {
+void launch_zero_window(int nf1, int nf2, int nf3, int x0, int x1, int y0, int y1, void *grid, int *dbg,
+                        cudaStream_t st) {
     const long long rows = (long long)(y1 - y0) * nf3;
     count_launch();
-    k_zero_window<T><<<grid_for(rows, 1), 256, 0, st>>>(nf1, nf2, x0, y0, x1 - x0, y1 - y0, rows,
-                                                        reinterpret_cast<C<T> *>(grid));
+    k_zero_window<T><<<grid_for(rows, 1), 256, 0, st>>>(nf1, nf2, nf3, x0, y0, x1 - x0, y1 - y0, rows,
+                                                        reinterpret_cast<C<T> *>(grid), dbg);
 }
 
 #define CURIG_INSTANTIATE(T)                                                                          \
@@ -2615,7 +2627,7 @@ void launch_zero_window(int nf1, int nf2, int nf3, int x0, int x1, int y0, int y
     template void launch_correct3_d2m<T>(const DevCorr &, const void *, void *, cudaStream_t);        \
     template void launch_cols_to_t<T>(int, int, int, int, const void *, void *, cudaStream_t);         \
     template void launch_t_to_grid<T>(int, int, int, int, const void *, void *, cudaStream_t);         \
-    template void launch_zero_window<T>(int, int, int, int, int, int, int, void *, cudaStream_t);      \
+    template void launch_zero_window<T>(int, int, int, int, int, int, int, void *, int *, cudaStream_t); \
     template void launch_zero_tpad<T>(int, int, int, int, void *, cudaStream_t);
 
 CURIG_INSTANTIATE(float)

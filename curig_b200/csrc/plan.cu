@@ -347,6 +347,13 @@ std::atomic<int> g_sparse_interp{-1};
 
 void set_sparse_interp(int n) { g_sparse_interp.store(n); }
 
+// The binning's limit, which a test lowers to bin a small call as a large one.
+namespace {
+std::atomic<long long> g_ranked_bytes{RANKED_BYTES};
+}
+
+void set_ranked_bytes(long long n) { g_ranked_bytes.store(n >= 0 ? n : RANKED_BYTES); }
+
 // ms2dirty's weighted gather takes a scratch vis * wgt from the pool, or, when
 // that allocation fails (or a test turns the scratch off), gathers vis and wgt
 // in one pass.
@@ -847,7 +854,7 @@ retry_tiles:
     p->d_scan = p->d_bcur + nb;
     CU_TRY(cudaMemsetAsync(p->d_kcount, 0, nkeys * sizeof(int), st));
     // few visibilities: their ranks now, records straight from input order later
-    const bool ranked = M * (7LL * esize) <= RANKED_BYTES;
+    const bool ranked = M * (7LL * esize) <= g_ranked_bytes.load();
     launch_bin_count(g, du, dv, dw, p->d_foc, p->d_keys_in, ranked ? p->d_tmp : nullptr, p->d_kcount, p->d_err, st);
     scan_ints(p->d_kcount, p->d_kcount, nkeys, false, p->d_scan, st);          // in place: first position per key
     launch_bins_from_keys(p->d_kcount, p->d_scan, nb, cbits, g.sub, p->d_bin_start, p->d_bin_count, p->d_nsub,
@@ -1005,7 +1012,8 @@ template <typename T>
 static int plane_fft(Plan *p, int dir, bool m2d) {
     const GridParams &gp = p->gp;
     const long long nx_rows = (long long)gp.nf2 * gp.nf3, ny_rows = (long long)p->ny * gp.nf3;
-    const FftGeom fg{p->nx, p->ny, gp.nf1, gp.nf2, gp.nf3, p->win_x[0], p->win_x[1], p->win_y[0], p->win_y[1]};
+    const FftGeom fg{p->nx, p->ny, gp.nf1, gp.nf2, gp.nf3, p->win_x[0], p->win_x[1], p->win_y[0], p->win_y[1],
+                     p->d_err};
     const char *twx = static_cast<const char *>(p->d_tw);
     const char *twy = twx ? twx + (size_t)p->fx.tw_len * 16 : nullptr;
     auto lib_x = [&] {
@@ -1041,7 +1049,8 @@ static cudaError_t zero_grid(Plan *p) {
     const double part = (double)(p->win_x[1] - p->win_x[0]) * (p->win_y[1] - p->win_y[0]) / ((double)gp.nf1 * gp.nf2);
     if (part > 0.85)
         return cudaMemsetAsync(p->d_grid, 0, (size_t)gp.nf1 * gp.nf2 * gp.nf3 * 2 * sizeof(T), p->st);
-    launch_zero_window<T>(gp.nf1, gp.nf2, gp.nf3, p->win_x[0], p->win_x[1], p->win_y[0], p->win_y[1], p->d_grid, p->st);
+    launch_zero_window<T>(gp.nf1, gp.nf2, gp.nf3, p->win_x[0], p->win_x[1], p->win_y[0], p->win_y[1], p->d_grid, p->d_err,
+                          p->st);
     return cudaSuccess;
 }
 

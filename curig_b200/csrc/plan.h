@@ -256,7 +256,8 @@ void launch_t_to_grid(int ny, int nf1, int nf2, int nf3, const void *t, void *gr
 template <typename T>
 void launch_zero_tpad(int nx, int ny, int nf2, int nf3, void *t, cudaStream_t st);
 template <typename T>
-void launch_zero_window(int nf1, int nf2, int nf3, int x0, int x1, int y0, int y1, void *grid, cudaStream_t st);
+void launch_zero_window(int nf1, int nf2, int nf3, int x0, int x1, int y0, int y1, void *grid, int *dbg,
+                        cudaStream_t st);
 // psi-hat of up to three axes (n3 = 0: two), one after the other in out
 void launch_psi_grids(int n1, int n2, int n3, int nq, const double *qx, const double *qg, double *out,
                       cudaStream_t st);
@@ -275,6 +276,9 @@ void set_gather_scratch(int on);
 // interpolator's sparse threshold of plans whose points are set afterwards
 // (negative: DEFAULT_SPARSE_I), for tests
 void set_sparse_interp(int n);
+// the binning's limit (RANKED_BYTES) for plans whose points are set afterwards
+// (negative: the default), for tests
+void set_ranked_bytes(long long n);
 // destroy the cached cuFFT handles no plan holds (returns how many); number cached
 int fft_cache_trim();
 int fft_cache_size();

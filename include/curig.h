@@ -253,6 +253,11 @@ void curig_test_gather_scratch(int on);
  * which curig_opts.sparse > 0 does not change.  No counterpart in the reference. */
 void curig_test_sparse_interp(int n);
 
+/* Test hook for the binning: plans whose points are set after this call place
+ * their records by ranks if these take at most n bytes, else by cursors as large
+ * calls do; n < 0 restores the default (112 MB).  No counterpart in the reference. */
+void curig_test_ranked_bytes(int64_t n);
+
 /* Generic NUFFT, types 1 (points -> modes) and 2 (modes -> points) in one or two
  * dimensions, on the w-free gridder (same kernel-width, grid-size and correction
  * rules as the gridder; takes the place of the reference's cunufft_setting /
