@@ -885,8 +885,9 @@ __device__ __forceinline__ int round_fix(float a, float k) {
 // three int32 planes.  Adding 1.5 * 2^70 rounds x to a multiple of 2^18 whose
 // quotient X = round(x / 2^18) is the bit-pattern difference (same binade for
 // |x| <= 2^54); h = X >> 18 and m = X & (2^18 - 1) split it further (m >= 0),
-// and the remainder x - X 2^18 (exact, |.| <= 2^17) is rounded to the integer
-// l by adding 1.5 * 2^52.  Four FP64 additions per term.  The chunk scale
+// and the remainder x - X 2^18 (|.| <= 2^17, one rounding) is rounded to the
+// integer l by adding 1.5 * 2^52.  Two FMAs and two additions per term, x = a k
+// itself unrounded.  The chunk scale
 // q = 2^k takes the largest k with max|c| wmax3 q <= 2^54, so |h| <= 2^18,
 // 0 <= m < 2^18, |l| <= 2^17 and, with at most 4096 terms per cell (sub <=
 // 4096), no plane's sum leaves int32: cell sums are exact and order-
@@ -924,7 +925,6 @@ k_spread_t(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__
     int *flr = fhr + ntile, *fhi = flr + ntile, *fli = fhi + ntile;
     int *fre = fhr, *fim = flr;                        // one-word planes: re, im
     float *colsum = reinterpret_cast<float *>(fhr + 2 * ntile);   // one-word: per start column sum|c|
-    // FP64 planes: re-high, im-high (int64, units of 2^18), re-low, im-low (int32)
     // FP64 planes: re high / mid / low, im high / mid / low (int32 each)
     int *hre = reinterpret_cast<int *>(smem), *mre = hre + ntile, *lre = mre + ntile;
     int *him = lre + ntile, *mim = him + ntile, *lim = mim + ntile;
@@ -1969,7 +1969,7 @@ __device__ __forceinline__ QuarterPix quarter(const DevCorr &cc, int r, int s) {
 // The transformed planes are read and written in the column-transposed
 // layout T[z][x'][y] (x' over the ny image columns in FFT order: grid column
 // x' for x' < ny - ny/2, nf1 - ny + x' above; y over nf2, contiguous), so the
-// y transforms are contiguous rows for cuFFT.  Thread index: r (the y side)
+// y transforms are contiguous rows.  Thread index: r (the y side)
 // fastest, so a warp's plane accesses are contiguous.
 
 // ms2dirty epilogue: w-screen sum over planes + all corrections, one pass.

@@ -164,8 +164,8 @@ int plan_execute(Plan *p, void *d_vis, const void *d_wgt, void *d_dirty, int typ
 int plan_execute_slabs(Plan *p, int type, void *d_vis, const void *d_wgt, void *d_dirty,
                        const cudaEvent_t *ready, const cudaEvent_t *done, int nev, bool prologue_done = false);
 constexpr int MAX_SLABS = 8;
-// Binning: bytes of records (28 per visibility in FP32, 52 in FP64) up to which
-// they go straight to their places from input order (they stay in the 126 MB
+// Binning: bytes of records (28 per visibility in FP32, 52 in FP64, counted as
+// 56) up to which they go straight to their places from input order (they stay in the 126 MB
 // L2).  Count + scatter + records against count with ranks + records, us, uv
 // tracks: FP32 2e5 61 -> 23, 2e6 170 -> 75, 4e6 255 -> 215, 8e6 446 -> 464;
 // FP64 2e5 45 -> 19, 2e6 142 -> 99, 4e6 230 -> 271.
