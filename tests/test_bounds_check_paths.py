@@ -3,7 +3,8 @@ the size of the call and of the grid: binning by ranks and by cursors (which lar
 calls take; curig_test_ranked_bytes lets small ones take them), with one and three
 row slabs; the row passes of every form (units that interleave or not, rows in
 two halves, partial windows of the grid, odd images) and the library's rows beside
-them; the third axis of the 3-D transform; the general tile kernels.
+them; the third axis of the 3-D transform; the general tile kernels; the
+interpolator's direct reads alone and not at all (curig_test_sparse_interp).
 
 The checked build must raise no flag and agree with the regular one: the order of
 the grid's additions differs, 1e-12 of the norm (FP64) and 1e-5 (FP32, as there)."""
@@ -28,7 +29,9 @@ BINNING = [(prec, nchan, slabs, limit) for prec in (0, 1) for nchan in (1, 3) fo
 GRIDS = [((64, 64), None, 0.2, {}), ((75, 53), None, 0.49, {}), ((33, 40), None, 0.3, {"bin_z": 2}),
          ((16, 20), (40, 48), 0.5, {}), ((15, 7), (1458, 1500), 0.1, {}), ((31, 20), (4608, 8192), 0.3, {}),
          ((16, 21), (6000, 64), 0.2, {}), ((15, 20), (64, 5000), 0.2, {}), ((24, 24), (2916, 4800), 0.3, {}),
-         ((16, 16), (10000, 40), 0.2, {}), ((40, 40), None, 0.3, {"eps": 1e-13})]
+         ((16, 16), (10000, 40), 0.2, {}), ((40, 40), None, 0.3, {"eps": 1e-13}),
+         ((64, 49), None, 0.49, {"direct": 1 << 30}), ((20, 21), (40, 48), 0.49, {"direct": 1 << 30}),
+         ((64, 49), None, 0.49, {"direct": 0, "bin_z": 2})]
 MODES = [(12, 10, 8), (31, 17, 40), (9, 20, 130)]
 
 
@@ -54,13 +57,14 @@ def binning(L, prec, nchan, slabs, limit):
     return d, v, np.array([launches])
 
 
-def planes(prec, image, grid, reach, opts):
+def planes(L, prec, image, grid, reach, opts):
     import torch
     from curig_b200 import GridderPlan
     ct = torch.complex64 if prec else torch.complex128
     nx, ny = image
     opts = dict(opts)
     eps = opts.pop("eps", 1e-5 if prec else 1e-9)
+    direct = opts.pop("direct", -1)               # the interpolator's threshold
     if grid:
         opts.update(w_term=1, grid_x=grid[0], grid_y=grid[1])
     rng = np.random.default_rng(nx + ny)
@@ -70,7 +74,11 @@ def planes(prec, image, grid, reach, opts):
     vis = rng.standard_normal((900, 1)) + 1j * rng.standard_normal((900, 1))
     img = rng.standard_normal((nx, ny)) + 1j * rng.standard_normal((nx, ny))
     p = GridderPlan(1, nx, ny, px, px, eps, precision="fp32" if prec else "fp64", accumulate=3, **opts)
-    p.setpts(torch.from_numpy(uvw).cuda(), freq)
+    L.lib.curig_test_sparse_interp(direct)
+    try:
+        p.setpts(torch.from_numpy(uvw).cuda(), freq)
+    finally:
+        L.lib.curig_test_sparse_interp(-1)
     d = torch.empty((nx, ny), dtype=ct, device="cuda")
     v = torch.empty((900, 1), dtype=ct, device="cuda")
     p.execute_dir(1, torch.from_numpy(vis).to(ct).cuda(), None, d)
@@ -109,7 +117,7 @@ def run_all(L):
         out["binning %s" % (case,)] = binning(L, *case)
     for prec in (0, 1):
         for case in GRIDS:
-            out["planes %d %s" % (prec, case)] = planes(prec, *case)
+            out["planes %d %s" % (prec, case)] = planes(L, prec, *case)
         for modes in MODES:
             out["volume %d %s" % (prec, modes)] = volume(L, prec, modes)
     return {"%s / %d" % (k, i): a for k, arrays in out.items() for i, a in enumerate(arrays)}
