@@ -996,13 +996,14 @@ k_spread_t(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__
         __syncthreads();
         // Scale statistics of the chunk: largest component of c (gathered into
         // bin order by k_vis_prep); one word: start-column histogram of it.
-        T m = 0;
+        T m = 0, bad = 0;                                // bad: NaN once a component is not finite
         if (fix || fix1 || fix64)
             for (int k = threadIdx.x; k < n; k += TTHREADS) {
                 const int i = start + k * stride;
                 const C<T> c = cs[i];
                 const T mc = fmax(fabs(c.x), fabs(c.y));
                 m = fmax(m, mc);
+                bad = fma(c.x, (T)0, fma(c.y, (T)0, bad));
                 if (fix1) {
                     const int cb = cell_bits(rec[i].w);
                     atomicAdd(colsum + ((cb >> 10) & 0x3ff) * tx + (cb & 0x3ff), (float)mc);
@@ -1011,12 +1012,15 @@ k_spread_t(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__
         T q = 1;
         double qinv = 1;
         if (fix || fix1 || fix64) {
+            if (bad != (T)0) m = (T)INFINITY;
             for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
             if (lane == 0) redbuf[warp] = m;
             __syncthreads();
             m = 0;
 #pragma unroll
             for (int w = 0; w < TWARPS; ++w) m = fmax(m, redbuf[w]);
+            const bool finite = m < (T)INFINITY;         // else NaN for the tile, as in k_spread_f32
+            if (!finite) m = 0;
             int k;
             if (fix) {
                 int e = m > (T)0 ? ilogb(m) + 1 : 0;       // 2^(e-1) <= m < 2^e
@@ -1042,12 +1046,12 @@ k_spread_t(DevGeom g, const int *__restrict__ bin_start, const int *__restrict__
                 for (int w = 0; w < TWARPS; ++w) bb = fmax(bb, redbuf[w]);
                 // float sums of <= 4096 terms: relative error < 2^-12, inside the bound's factor-2 margin
                 int em = m > (T)0 ? ilogb(m * g.wmax3) + 1 : 0;
-                int es = bb > (T)0 ? ilogb(bb * g.wmax3) + 1 : 0;
+                int es = finite && bb > (T)0 ? ilogb(bb * g.wmax3) + 1 : 0;
                 k = min(22 - em, 30 - es);
             }
             k = min(k, 120);                             // chunks of near-zero values
             q = (T)ldexp(1.0, k);
-            qinv = ldexp(1.0, -k);
+            qinv = finite ? ldexp(1.0, -k) : NAN;
         }
         __syncthreads();
         // Lane l of a warp takes row l of the 32 x L matrix of the chunk's
@@ -1455,7 +1459,7 @@ k_spread_f32(DevGeom g, const int *__restrict__ bin_start, const int *__restrict
         __syncthreads();
         // chunk statistics: largest component of c, one word: start-column sums
         // (four elements per thread in flight: the loads are issued first)
-        float m = 0.f;
+        float m = 0.f, bad = 0.f;                        // bad: NaN once a component is not finite
         if (fixed)
             for (int k0 = threadIdx.x; k0 < n; k0 += 4 * TTHREADS) {
                 float2 cc[4];
@@ -1475,6 +1479,7 @@ k_spread_f32(DevGeom g, const int *__restrict__ bin_start, const int *__restrict
                 for (int u = 0; u < 4; ++u) {
                     const float mc = fmaxf(fabsf(cc[u].x), fabsf(cc[u].y));
                     m = fmaxf(m, mc);
+                    bad = fmaf(cc[u].x, 0.f, fmaf(cc[u].y, 0.f, bad));
                     if (one && k0 + u * TTHREADS < n &&
                         IN_BOUNDS(((cb[u] >> 10) & 0x3ff) < g.ty && (cb[u] & 0x3ff) < tx, g.dbg))
                         atomicAdd(colsum + ((cb[u] >> 10) & 0x3ff) * tx + (cb[u] & 0x3ff), mc);
@@ -1484,12 +1489,17 @@ k_spread_f32(DevGeom g, const int *__restrict__ bin_start, const int *__restrict
         float q = 1.f;
         double qinv = 1.0;
         if (fixed) {
+            if (bad != 0.f) m = INFINITY;
             for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
             if (lane == 0) redbuf[warp] = m;
             __syncthreads();
             m = 0.f;
 #pragma unroll
             for (int w = 0; w < TWARPS; ++w) m = fmaxf(m, redbuf[w]);
+            // A value that is not finite would leave the integers as a finite
+            // one: its chunk adds NaN to its tile's cells instead.
+            const bool finite = m < INFINITY;
+            if (!finite) m = 0.f;
             int k;
             if (two) {
                 int e = m > 0.f ? ilogb(m) + 1 : 0;       // 2^(e-1) <= m < 2^e
@@ -1530,12 +1540,12 @@ k_spread_f32(DevGeom g, const int *__restrict__ bin_start, const int *__restrict
 #pragma unroll
                 for (int w = 0; w < TWARPS; ++w) bb = fmaxf(bb, redbuf[w]);
                 const int em = m > 0.f ? ilogb(m * g.wmax3) + 1 : 0;
-                const int es = bb > 0.f ? ilogb(bb * g.wzmax) + 1 : 0;
+                const int es = finite && bb > 0.f ? ilogb(bb * g.wzmax) + 1 : 0;
                 k = min(22 - em, 30 - es);
             }
             k = min(k, 120);
             q = (float)ldexp(1.0, k);
-            qinv = ldexp(1.0, -k);
+            qinv = finite ? ldexp(1.0, -k) : NAN;
         }
         __syncthreads();
         // class schedule: lane k + 16 f, element 2t + f of class k at step t;
