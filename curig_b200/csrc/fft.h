@@ -43,7 +43,9 @@ bool fft_make_plan(int n, int esize, FftPlan &p);
 struct FftGeom {
     int nx, ny, nf1, nf2, nf3;
     int x0, x1, y0, y1;            // window of the grid that the points reach (even bounds)
-    int *dbg;                      // bounds-checked build: error flags raised by the index checks
+#ifdef CURIG_BOUNDS_CHECK
+    int *dbg;                      // error flags raised by the index checks
+#endif
 };
 
 // Twiddle tables of both plans (either may be empty), x first, in the plan's precision.

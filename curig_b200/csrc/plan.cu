@@ -1012,8 +1012,10 @@ template <typename T>
 static int plane_fft(Plan *p, int dir, bool m2d) {
     const GridParams &gp = p->gp;
     const long long nx_rows = (long long)gp.nf2 * gp.nf3, ny_rows = (long long)p->ny * gp.nf3;
-    const FftGeom fg{p->nx, p->ny, gp.nf1, gp.nf2, gp.nf3, p->win_x[0], p->win_x[1], p->win_y[0], p->win_y[1],
-                     p->d_err};
+    FftGeom fg{p->nx, p->ny, gp.nf1, gp.nf2, gp.nf3, p->win_x[0], p->win_x[1], p->win_y[0], p->win_y[1]};
+#ifdef CURIG_BOUNDS_CHECK
+    fg.dbg = p->d_err;
+#endif
     const char *twx = static_cast<const char *>(p->d_tw);
     const char *twy = twx ? twx + (size_t)p->fx.tw_len * 16 : nullptr;
     auto lib_x = [&] {
